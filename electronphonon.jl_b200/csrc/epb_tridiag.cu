@@ -263,24 +263,31 @@ __device__ __forceinline__ void load_rows(const TriArgs& a, int64_t b, int lane,
   }
 }
 
-// MODE 0: window band ranges from Sturm counts at the shifts; MODE 1: all eigenvalues; MODE 2: the
-// tridiagonal itself (d, e^2) for a later per-band bisection.
 // Number of sign changes of the Sturm sequence p_i = (d_i - sigma) p_{i-1} - e_{i-1}^2 p_{i-2} of a tridiagonal
-// scaled to norm <= 1, i.e. of eigenvalues below sigma: a zero takes the sign opposite to its predecessor's (the
-// quotient form's -pivmin). No division on the chain: 53 bisection steps of order 8 take a fifth of the quotients'
-// time. |p_i| <= 3^i; small ones are lifted out of the underflow range every eighth step.
+// scaled to norm <= 1, i.e. of eigenvalues below sigma. No division on the chain: 53 bisection steps of order 8 take a
+// fifth of the quotients' time. Every e^2 is zero or at least STURM_E2 (the caller sees to it).
+// A zero p_i takes the sign opposite to its predecessor's; the next one is -e_i^2 p_{i-1} with that sign, so one change
+// is counted. Where e_i^2 is zero nothing of the block above reaches p_{i+1}, and after a zero p_i the recurrence would
+// stay at zero for good: the row starts a block of its own, p_{i+1} = d_{i+1} - sigma after a one.
+// |p_i| <= 3^i. The larger of two neighbours falls by at most STURM_E2 / 2 a step, so lifting both every fourth step
+// keeps them out of the underflow range.
+constexpr double STURM_E2 = 0x1p-120;
 __device__ __forceinline__ int sturm_signs(const double* d, const double* e2, int n, double sigma) {
   double p1 = 1.0, p = d[0] - sigma;
   bool neg = !(p > 0.0);
   int c = neg;
   for (int i = 1; i < n; ++i) {
-    const double t = fma(d[i] - sigma, p, -(e2[i - 1] * p1));
-    p1 = p;
+    const double b = e2[i - 1];
+    const bool first = b == 0.0;
+    const double q = first ? 1.0 : p;
+    const double t = fma(d[i] - sigma, q, -(b * p1));
+    neg = neg && !first;
+    p1 = q;
     p = t;
     const bool ng = t < 0.0 || (t == 0.0 && !neg);
     c += ng != neg;
     neg = ng;
-    if ((i & 7) == 0 && fmax(fabs(p), fabs(p1)) < 0x1p-300) {
+    if ((i & 3) == 0 && fmax(fabs(p), fabs(p1)) < 0x1p-300) {
       p *= 0x1p600;
       p1 *= 0x1p600;
     }
@@ -349,7 +356,8 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
       const double sc = ldexp(1.0, -ex);
       __syncwarp();
       s.d[lane] *= sc;
-      s.e2[lane] *= sc * sc;
+      const double es = s.e2[lane] * sc * sc;
+      s.e2[lane] = es < STURM_E2 ? 0.0 : es;  // |e| < 2^-60 of the norm: below a hundredth of its last bit
       __syncwarp();
       const double eps = 2.220446049250313e-16;
       double lo = lane < n ? s.d[lane] - rad * sc : 0.0, hi = lane < n ? s.d[lane] + rad * sc : 0.0;
@@ -358,8 +366,10 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
         lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       }
-      lo -= 4 * eps;
-      hi += 4 * eps;
+      if (span > 0.0) {  // the zero matrix keeps [0, 0]
+        lo -= 4 * eps;
+        hi += 4 * eps;
+      }
       if (lane < n && live) {
         for (int it = 0; it < 200; ++it) {
           const double mid = 0.5 * (lo + hi);
