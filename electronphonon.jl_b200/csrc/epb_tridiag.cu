@@ -123,8 +123,9 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
     const T a2 = x1r * x1r + x1i * x1i;
     const T rx = tri_rsqrt(xn2 == T(0) ? T(1) : xn2), ra = tri_rsqrt(a2 == T(0) ? T(1) : a2);
     const T xn = xn2 * rx, a1 = a2 * ra;
-    // a column that is already reduced (xn2 = 0) takes beta = 0: nothing changes
-    const T beta = xn2 == T(0) ? T(0) : T(1) / fma(xn, a1, xn2);
+    // a column that is already reduced takes beta = 0: nothing changes. In FP64 so does one so short that 1 / xn2 would
+    // leave the range of a double.
+    const T beta = xn2 <= (sizeof(T) == 8 ? T(1e-290) : T(0)) ? T(0) : T(1) / fma(xn, a1, xn2);
     T ur = T(0), ui = T(0);
     if (lane > k + 1) {
       ur = xr;
@@ -351,8 +352,12 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
       double span = lane < n ? fabs(s.d[lane]) + rad : 0.0;
 #pragma unroll
       for (int o = N / 2; o > 0; o >>= 1) span = fmax(span, __shfl_xor_sync(0xffffffffu, span, o));
+      // An infinity or NaN of the matrix is one in its column's length, hence in T (fmax above drops NaN): no energies.
+      const unsigned odd = __ballot_sync(0xffffffffu, lane < n && !(isfinite(s.d[lane]) && isfinite(s.e2[lane])));
+      const bool bad = (odd >> (N * g) & (0xffffffffu >> (32 - N))) != 0 || !isfinite(span);
       int ex = 0;
-      if (span > 0.0 && span < 1e300) frexp(span, &ex);
+      if (span > 0.0 && !bad) frexp(span, &ex);
+      ex = max(ex, -500);  // below, squares underflow anyway, and sc would overflow
       const double sc = ldexp(1.0, -ex);
       __syncwarp();
       s.d[lane] *= sc;
@@ -360,18 +365,19 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
       s.e2[lane] = es < STURM_E2 ? 0.0 : es;  // |e| < 2^-60 of the norm: below a hundredth of its last bit
       __syncwarp();
       const double eps = 2.220446049250313e-16;
-      double lo = lane < n ? s.d[lane] - rad * sc : 0.0, hi = lane < n ? s.d[lane] + rad * sc : 0.0;
+      // padding rows do not widen the interval
+      double lo = lane < n ? s.d[lane] - rad * sc : 1.0, hi = lane < n ? s.d[lane] + rad * sc : -1.0;
 #pragma unroll
       for (int o = N / 2; o > 0; o >>= 1) {
         lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       }
       if (span > 0.0) {  // the zero matrix keeps [0, 0]
-        lo -= 4 * eps;
+      lo -= 4 * eps;
         hi += 4 * eps;
       }
       if (lane < n && live) {
-        for (int it = 0; it < 200; ++it) {
+        for (int it = bad ? 200 : 0; it < 200; ++it) {
           const double mid = 0.5 * (lo + hi);
           if (!(hi - lo > 2 * eps * fmax(fabs(lo), fabs(hi))) || mid <= lo || mid >= hi) break;
           if (sturm_signs(s.d, s.e2, n, mid) > lane)
@@ -379,7 +385,7 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
           else
             lo = mid;
         }
-        a.E[b * (int64_t)n + lane] = ldexp(0.5 * (lo + hi), ex);
+        a.E[b * (int64_t)n + lane] = bad ? nan("") : ldexp(0.5 * (lo + hi), ex);
       }
     }
     __syncwarp();

@@ -64,3 +64,29 @@ def test_states_and_bands(n):
         assert _worst(B.host(bands.eigvals(x)).T, np.stack([h, h])) <= 10 * n * EPS
         assert _worst(B.host(bands.eigvals(x, prec=L.PREC_MIXED)).T, np.stack([h, h])) <= 1e-5
         bands.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 5, 8, 11, 16, 17, 32])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_not_finite(n, bad):
+    """A matrix with a NaN or infinity gets no energies, wherever the entry is; its neighbours in the batch keep
+    theirs, at any scale whose squares a double holds."""
+    from epb200 import batched as B
+
+    rng = np.random.default_rng(n)
+    hs = rng.standard_normal((9, n, n)) + 1j * rng.standard_normal((9, n, n))
+    hs = hs + hs.conj().transpose(0, 2, 1)
+    hs[0] = np.diag(np.arange(n)) + 1e-155 * hs[0]  # columns whose squared length has no reciprocal
+    hs[1] *= 1e-140
+    hs[3] *= 1e140
+    given = hs.copy()
+    for k, (i, j) in {2: (0, n - 1), 4: (0, 0), 6: (n - 1, n - 1), 7: (n // 2, n - 1)}.items():
+        given[k, i, j] = bad
+    hit = np.array([k in (2, 4, 6, 7) for k in range(9)])
+    e = B.host(B.eigvals_batched(B.jl(np.asfortranarray(given.transpose(1, 2, 0))))).T
+    assert np.isnan(e[hit]).all()
+    assert _worst(e[~hit], hs[~hit]) <= 10 * n * EPS
+    tiny = np.asfortranarray((1e-170 * hs[5:6]).transpose(1, 2, 0))  # squares underflow: at least of its own size
+    e = B.host(B.eigvals_batched(B.jl(tiny)))
+    assert np.isfinite(e).all() and np.abs(e).max() <= 2 * n * np.abs(tiny).max()
