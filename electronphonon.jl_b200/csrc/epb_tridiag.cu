@@ -74,8 +74,17 @@ __device__ __forceinline__ void tri_pick(float& v, float x, int j, int k) {
   asm("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %2, %3;\n\t@p mov.f32 %0, %1;\n\t}" : "+f"(v) : "f"(x), "r"(j), "r"(k));
 }
 
-__device__ __forceinline__ double tri_rsqrt(double x) { return rsqrt(x); }
-__device__ __forceinline__ float tri_rsqrt(float x) { return rsqrtf(x); }
+// Square root of x2 and its reciprocal (1 for zero). FP64 takes one reciprocal square root, good to an ulp, for a square
+// root and a division; the FP32 one is good to two only, so FP32 takes the square root and divides.
+__device__ __forceinline__ double tri_root(double x2, double& inv) {
+  inv = rsqrt(x2 == 0.0 ? 1.0 : x2);
+  return x2 * inv;
+}
+__device__ __forceinline__ float tri_root(float x2, float& inv) {
+  const float x = sqrtf(x2);
+  inv = 1.f / (x2 == 0.f ? 1.f : x);
+  return x;
+}
 
 __device__ __forceinline__ double sturm_div(double a, double b) { return a / b; }
 // FP32 counts are only used with guard intervals far wider than the 2-ulp fast division error.
@@ -121,8 +130,8 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
     if (k == N - 2) break;      // last off-diagonal: no reflection left to apply
     const T x1r = __shfl_sync(0xffffffffu, xr, k + 1, N), x1i = __shfl_sync(0xffffffffu, xi, k + 1, N);
     const T a2 = x1r * x1r + x1i * x1i;
-    const T rx = tri_rsqrt(xn2 == T(0) ? T(1) : xn2), ra = tri_rsqrt(a2 == T(0) ? T(1) : a2);
-    const T xn = xn2 * rx, a1 = a2 * ra;
+    T rx, ra;
+    const T xn = tri_root(xn2, rx), a1 = tri_root(a2, ra);
     // a column that is already reduced takes beta = 0: nothing changes. In FP64 so does one so short that 1 / xn2 would
     // leave the range of a double.
     const T beta = xn2 <= (sizeof(T) == 8 ? T(1e-290) : T(0)) ? T(0) : T(1) / fma(xn, a1, xn2);
@@ -168,8 +177,8 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
     // column k + 1 after the update, its squared length below the diagonal summed in the gaps of the update
     {
       const auto uj = s.u[k + 1], wj = s.w[k + 1];
-      nr = fma(-wi, uj.y, fma(-wr, uj.x, fma(-ui, wj.y, fma(-ur, wj.x, nr))));
-      ni = fma(wr, uj.y, fma(-wi, uj.x, fma(ur, wj.y, fma(-ui, wj.x, ni))));
+      nr -= fma(wi, uj.y, fma(wr, uj.x, fma(ui, wj.y, ur * wj.x)));
+      ni -= fma(-wr, uj.y, fma(wi, uj.x, fma(-ur, wj.y, ui * wj.x)));
     }
     xr = nr;  // the next step's column
     xi = ni;
@@ -186,9 +195,11 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
         }
       if (j > k) {
         const auto uj = s.u[j], wj = s.w[j];
-        // A[i][j] -= u_i conj(w_j) + w_i conj(u_j); u_i = w_i = 0 for rows i <= k
-        ar[j] = fma(-wi, uj.y, fma(-wr, uj.x, fma(-ui, wj.y, fma(-ur, wj.x, ar[j]))));
-        ai[j] = fma(wr, uj.y, fma(-wi, uj.x, fma(ur, wj.y, fma(-ui, wj.x, ai[j]))));
+        // A[i][j] -= u_i conj(w_j) + w_i conj(u_j); u_i = w_i = 0 for rows i <= k. The four products are summed first:
+        // one rounding at the size of A (four FMAs onto A: eigenvalues of order 8 off by 0.43 eps of the norm in rms
+        // instead of 0.35, of order 24 by 0.172 instead of 0.163).
+        ar[j] -= fma(wi, uj.y, fma(wr, uj.x, fma(ui, wj.y, ur * wj.x)));
+        ai[j] -= fma(-wr, uj.y, fma(wi, uj.x, fma(-ur, wj.y, ui * wj.x)));
       }
     }
     xn2 += other;
