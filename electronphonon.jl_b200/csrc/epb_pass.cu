@@ -270,14 +270,15 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
   // second captures the pass (status checks left out of the graph), later ones replay it.
   PassGraph& pg = m->graph;
   const PassKey key{xk, nk, xq, nq, prec, k_batch, sample_stride, ek_out, omega_out, g2sum_out, g2_sample, ch.rot, ch.kq};
-  if (pg.exec && pg.key == key) {
+  if (!(pg.key == key)) {  // a graph of other arguments
+    if (pg.exec) cudaGraphExecDestroy(pg.exec);
+    pg.exec = nullptr;
+    pg.warm = false;
+  }
+  if (pg.exec) {
     EPB_CUDA(cudaGraphLaunch(pg.exec, ctx->stream));
     ctx->launches += pg.launches;
-  } else if (pg.warm && pg.key == key) {
-    if (pg.exec) {
-      cudaGraphExecDestroy(pg.exec);
-      pg.exec = nullptr;
-    }
+  } else if (pg.warm) {
     cudaGraph_t graph = nullptr;
     const int64_t l0 = ctx->launches;
     EPB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
