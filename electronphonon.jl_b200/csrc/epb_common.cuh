@@ -117,6 +117,8 @@ struct epb_ctx {
   int cc_major = 0, cc_minor = 0;
   void* ws[EPB_WS_NSLOTS] = {};
   size_t ws_bytes[EPB_WS_NSLOTS] = {};
+  uint64_t ws_moves = 0;     // times a workspace got another address
+  bool own_capture = false;  // the capture in progress is epb_eph_pass's, which looks at ws_moves before a replay
   int fail_alloc_nth = 0;  // test hook
   // Small pinned host scratch for scalar read-backs.
   int64_t* pinned = nullptr;
@@ -165,6 +167,7 @@ struct epb_rset {
 // A model's hot-path operators (caller-owned device memory) plus the library's derived data.
 // Arguments a captured pass was recorded with (a replay is valid only for the same buffers and sizes).
 struct PassKey {
+  const epb_ctx* ctx = nullptr;  // whose workspaces and status words the graph uses
   const void* xk = nullptr;
   int64_t nk = 0;
   const void* xq = nullptr;
@@ -174,13 +177,14 @@ struct PassKey {
   const void *ek = nullptr, *om = nullptr, *g2 = nullptr, *samp = nullptr;
   int rot = 0, kq = 1;  // rotation kernel and kR->kq form the graph was captured with
   bool operator==(const PassKey& o) const {
-    return xk == o.xk && nk == o.nk && xq == o.xq && nq == o.nq && prec == o.prec && k_batch == o.k_batch &&
+    return ctx == o.ctx && xk == o.xk && nk == o.nk && xq == o.xq && nq == o.nq && prec == o.prec && k_batch == o.k_batch &&
            stride == o.stride && ek == o.ek && om == o.om && g2 == o.g2 && samp == o.samp && rot == o.rot && kq == o.kq;
   }
 };
 struct PassGraph {
   PassKey key;
   bool warm = false;                 // one eager run with `key` has sized the workspaces
+  uint64_t ws_moves = 0;             // the context's count after that run
   cudaGraphExec_t exec = nullptr;    // the captured pass for `key`
   int64_t launches = 0;              // kernels in the graph
 };
@@ -214,7 +218,8 @@ void prof_end(epb_ctx* ctx);
 // Grow-only workspace slot; returns EPB_ERR_OOM on failure.
 int ws_get(epb_ctx* ctx, int slot, size_t bytes, void** out);
 // The same for an optional workspace: EPB_ERR_UNSUPPORTED when it would have to grow and cannot (no memory, or the
-// stream is being captured).
+// stream is being captured), and under a capture that is not the library's own, whose graph would keep an address that
+// the next growth frees.
 int ws_try(epb_ctx* ctx, int slot, size_t bytes, void** out);
 int make_current(epb_ctx* ctx);
 

@@ -43,6 +43,7 @@ int ws_get(epb_ctx* ctx, int slot, size_t bytes, void** out) {
     }
     ctx->ws[slot] = nullptr;
     ctx->ws_bytes[slot] = 0;
+    ++ctx->ws_moves;
   }
   size_t want = bytes + bytes / 8;  // headroom so that slowly growing callers do not churn
   void* p = nullptr;
@@ -54,18 +55,21 @@ int ws_get(epb_ctx* ctx, int slot, size_t bytes, void** out) {
   }
   ctx->ws[slot] = p;
   ctx->ws_bytes[slot] = want;
+  ++ctx->ws_moves;
   *out = p;
   return EPB_OK;
 }
 
+// Whether the context's stream is being captured (or cannot be asked).
+static bool capturing(epb_ctx* ctx) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 int ws_try(epb_ctx* ctx, int slot, size_t bytes, void** out) {
-  if (ctx->ws_bytes[slot] < bytes) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      return EPB_ERR_UNSUPPORTED;
-    }
-  }
+  if (capturing(ctx) && (!ctx->own_capture || ctx->ws_bytes[slot] < bytes)) return EPB_ERR_UNSUPPORTED;
   const int st = ws_get(ctx, slot, bytes, out);
   if (st != EPB_ERR_OOM) return st;
   clear_error();

@@ -269,8 +269,10 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
   // Graph mode: the first call with these arguments runs eagerly (sizing every workspace), the
   // second captures the pass (status checks left out of the graph), later ones replay it.
   PassGraph& pg = m->graph;
-  const PassKey key{xk, nk, xq, nq, prec, k_batch, sample_stride, ek_out, omega_out, g2sum_out, g2_sample, ch.rot, ch.kq};
-  if (!(pg.key == key)) {  // a graph of other arguments
+  const PassKey key{ctx, xk, nk, xq, nq, prec, k_batch, sample_stride, ek_out, omega_out, g2sum_out, g2_sample, ch.rot,
+                    ch.kq};
+  // a graph of other arguments, or one that holds the address of a workspace that has moved since
+  if (!(pg.key == key) || pg.ws_moves != ctx->ws_moves) {
     if (pg.exec) cudaGraphExecDestroy(pg.exec);
     pg.exec = nullptr;
     pg.warm = false;
@@ -282,8 +284,10 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
     cudaGraph_t graph = nullptr;
     const int64_t l0 = ctx->launches;
     EPB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    ctx->own_capture = true;
     int st = eph_pass_run(ctx, m, xk, nk, xq, nq, prec, k_batch, sample_stride, ek_out, omega_out, g2sum_out, g2_sample,
                           nullptr, true);
+    ctx->own_capture = false;
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
     pg.launches = ctx->launches - l0;
     ctx->launches = l0;
@@ -302,6 +306,7 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
                           nullptr);
     if (st != EPB_OK) return st;
     pg.key = key;
+    pg.ws_moves = ctx->ws_moves;
     pg.warm = true;
   }
   EPB_TRY(eigh_check(ctx));

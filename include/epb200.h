@@ -373,8 +373,9 @@ EPB_API int epb_model_destroy(epb_model* model);
    _loop_eph_over_k_and_kq_batched (src/calculator/run_eph_over_k_and_kq.jl:792-892). */
 /* Graph mode (off by default): epb_eph_pass runs the first call with a given argument set eagerly,
    captures the second as a CUDA graph and replays it on later calls with the same buffers and sizes
-   (the production loop refills the same device buffers). Ignored on the legacy default stream and
-   while profiling. */
+   (the production loop refills the same device buffers). A call that moves a workspace of the context in
+   between (a larger one of any kind) starts this over. Ignored on the legacy default stream and while
+   profiling. */
 EPB_API int epb_set_graph_mode(epb_ctx* ctx, int on);
 /* Rotation kernel of the mixed pass for nw = 16, nm = 12 (the fused rotation of
    ext/ElectronPhononCUDAExt.jl:146-201 and its two-GEMM fallback): 0 = warp-level tensor cores,

@@ -53,3 +53,77 @@ def test_two_sets_of_buffers(graph_mode):
         for a, b in zip(_arrays(outs[which]), ref[which]):
             np.testing.assert_array_equal(a, b)
     dm.close()
+
+
+def _grow(nw, nm, n_el, nk):
+    """Larger calls on the same context: the scratch of the FP64 Fourier sums and of RR -> kR moves."""
+    import torch
+
+    from epb200 import batched as B
+    from epb200.wannier import WannierObject, to_device
+
+    rng = np.random.default_rng(nk)
+    irvec, ir_ep = synth.irvec_box(n_el), synth.irvec_box(1)
+    op = rng.standard_normal((nw * nw * nm * len(ir_ep), len(irvec))) + 0j
+    obj = to_device(WannierObject(irvec, np.asfortranarray(op), irvec_next=ir_ep))
+    x = np.asfortranarray(rng.random((3, nk)))
+    itp = B.get_interpolator(obj)
+    B.get_fourier_batched(itp, x)
+    uks = B.jl(np.repeat(np.eye(nw, dtype=complex)[:, :, None], nk, axis=2))
+    B.get_eph_RR_to_kR_batched(B.jl_empty((nw * nw * nm, len(ir_ep), nk), torch.complex128), itp, x, uks)
+
+
+@pytest.mark.gpu
+def test_workspaces_that_move(graph_mode):
+    """Larger calls between captured passes move the scratch that the graph has the address of: the pass runs again
+    on the new one. Sizes at which the FP64 vertex product keeps its operands in that scratch."""
+    from epb200 import pipeline as P
+    from epb200.batched import jl
+
+    dm = P.DeviceModel(synth.config2_model(seed=4, n_el=1, n_ph=2, nw=16, natom=4))
+    xk, xq = jl(synth.random_kpoints(3, 30)), jl(synth.random_kpoints(4096, 31))
+    graph_mode.set_graph_mode(False)
+    ref = _arrays(_run(P, dm, xk, xq, k_batch=2))
+    graph_mode.set_graph_mode(True)
+    out, held = None, []
+    for grow in (0, 0, 0, 600, 0, 0, 2500, 0, 0):
+        if grow:
+            _grow(8, 6, 2, grow)
+        held.append(graph_mode.workspace_bytes())
+        if out is not None:
+            for t in (out.ek, out.omega, out.g2_sample):
+                t.fill_(-1)
+        out = _run(P, dm, xk, xq, out, k_batch=2)
+        for a, b in zip(_arrays(out), ref):
+            np.testing.assert_array_equal(a, b)
+    assert held[3] > held[2] and held[6] > held[5]  # the calls in between did grow them
+    dm.close()
+
+
+@pytest.mark.gpu
+def test_sum_in_a_callers_graph(graph_mode):
+    """A large FP64 Fourier sum in a graph that the caller captures uses none of the context's scratch: it replays
+    after larger calls have moved that."""
+    import torch
+
+    from epb200 import batched as B
+    from epb200.wannier import WannierObject, to_device
+
+    rng = np.random.default_rng(1)
+    irvec = synth.irvec_box(2)
+    op = rng.standard_normal((1500, len(irvec))) + 1j * rng.standard_normal((1500, len(irvec)))
+    itp = B.get_interpolator(to_device(WannierObject(irvec, np.asfortranarray(op))))
+    x = B.jl(np.asfortranarray(rng.random((3, 3000))))
+    out = B.jl_empty((1500, 3000), torch.complex128)
+    eager = B.get_fourier_batched(itp, x).clone()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        B.get_fourier_batched(itp, x, out=out)
+    _grow(8, 6, 2, 2500)
+    bar = 2 * (len(irvec) + 16) * np.finfo(np.float64).eps * np.abs(op).sum(axis=1).max()
+    for _ in range(2):
+        out.fill_(-1)
+        g.replay()
+        assert (out - eager).abs().max().item() <= bar
+    del g
