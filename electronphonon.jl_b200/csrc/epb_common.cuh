@@ -118,6 +118,8 @@ struct epb_ctx {
   void* ws[EPB_WS_NSLOTS] = {};
   size_t ws_bytes[EPB_WS_NSLOTS] = {};
   uint64_t ws_moves = 0;     // times a workspace got another address
+  // recorded behind the last use of scratch that calls on different streams share (scratch_begin, scratch_end)
+  cudaEvent_t scratch_ev = nullptr;
   bool own_capture = false;  // the capture in progress is epb_eph_pass's, which looks at ws_moves before a replay
   int fail_alloc_nth = 0;  // test hook
   // Small pinned host scratch for scalar read-backs.
@@ -221,6 +223,14 @@ int ws_get(epb_ctx* ctx, int slot, size_t bytes, void** out);
 // stream is being captured), and under a capture that is not the library's own, whose graph would keep an address that
 // the next growth frees.
 int ws_try(epb_ctx* ctx, int slot, size_t bytes, void** out);
+// Brackets around work that keeps something in the context's memory between its kernels without a wait of the host at
+// its end: a caller that moves the context to another stream (epb_set_stream) orders nothing itself, so such work waits
+// for the last of its kind, on whichever stream that ran. Nothing is recorded under a capture, whose work runs later:
+// epb_eph_pass brackets the launch of its graph.
+int scratch_begin(epb_ctx* ctx);
+int scratch_end(epb_ctx* ctx);
+// Whether the context's stream is being captured (or cannot be asked).
+bool capturing(epb_ctx* ctx);
 int make_current(epb_ctx* ctx);
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -60,8 +60,7 @@ int ws_get(epb_ctx* ctx, int slot, size_t bytes, void** out) {
   return EPB_OK;
 }
 
-// Whether the context's stream is being captured (or cannot be asked).
-static bool capturing(epb_ctx* ctx) {
+bool capturing(epb_ctx* ctx) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
   cudaGetLastError();
@@ -74,6 +73,19 @@ int ws_try(epb_ctx* ctx, int slot, size_t bytes, void** out) {
   if (st != EPB_ERR_OOM) return st;
   clear_error();
   return EPB_ERR_UNSUPPORTED;
+}
+
+int scratch_begin(epb_ctx* ctx) {
+  if (!ctx->scratch_ev || capturing(ctx)) return EPB_OK;
+  EPB_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->scratch_ev, 0));
+  return EPB_OK;
+}
+
+int scratch_end(epb_ctx* ctx) {
+  if (capturing(ctx)) return EPB_OK;
+  if (!ctx->scratch_ev) EPB_CUDA(cudaEventCreateWithFlags(&ctx->scratch_ev, cudaEventDisableTiming));
+  EPB_CUDA(cudaEventRecord(ctx->scratch_ev, ctx->stream));
+  return EPB_OK;
 }
 
 // The side stream and its events (non-blocking stream, timing-free events), created once.
@@ -208,6 +220,10 @@ int epb_destroy(epb_ctx* ctx) {
   }
   for (auto& e : ctx->side_ev)
     if (e) cudaEventDestroy(e);
+  if (ctx->scratch_ev) {
+    cudaEventSynchronize(ctx->scratch_ev);  // the last use may have been on another stream
+    cudaEventDestroy(ctx->scratch_ev);
+  }
   if (ctx->tail) {
     cudaStreamSynchronize(ctx->tail);
     cudaStreamDestroy(ctx->tail);

@@ -56,8 +56,8 @@ __device__ __forceinline__ bool eigh_skip(const EighArgs& a, int n, int nmax, in
   return true;
 }
 
-// FP64: one CTA of NT threads per matrix at a time, taken from a device work counter. Only the upper triangle of A is
-// kept. A round is two phases with a barrier after each:
+// FP64: one CTA of NT threads per matrix at a time, taken from a device work counter (without one: in turn).
+// Only the upper triangle of A is kept. A round is two phases with a barrier after each:
 //   1  a thread per pair forms its rotation and its own 2 x 2 block (a_pq = 0); all apply the previous round's
 //      rotations to V
 //   2  a thread per unordered couple of pairs takes the four elements where they cross, applies the column and the row
@@ -107,10 +107,13 @@ __global__ void __launch_bounds__(NT, MINB) eigh64_kernel(EighArgs a, unsigned l
   long long* next = reinterpret_cast<long long*>(flag + 2);
   const int tid = threadIdx.x, lane = tid & 31;
 
-  for (;;) {
-    if (tid == 0) *next = (long long)atomicAdd(counter, 1ull);
-    __syncthreads();
-    const int64_t b = *next;
+  for (int64_t turn = blockIdx.x;; turn += gridDim.x) {
+    int64_t b = turn;
+    if (counter) {
+      if (tid == 0) *next = (long long)atomicAdd(counter, 1ull);
+      __syncthreads();
+      b = *next;
+    }
     if (b >= a.batch) break;
     const int n = a.nvec ? a.nvec[b] : a.n_uniform;
     if (eigh_skip(a, n, NMAX, tid)) {
@@ -513,7 +516,8 @@ static int launch_eigh(epb_ctx* ctx, Kern kern, size_t smem, int threads, EighAr
   return EPB_OK;
 }
 
-// One FP64 instance over the batch: its work counter is a context word of its own (status words 28, 29).
+// One FP64 instance over the batch. Its work counter is a context word that calls on other streams share; a captured
+// launch, which may be replayed beside them, goes without.
 template <int NMAX, int NT, int MINB>
 static int launch_eigh64(epb_ctx* ctx, EighArgs& a) {
   constexpr int smem = Eigh64Smem<NMAX, NT>::TOTAL;
@@ -524,14 +528,15 @@ static int launch_eigh64(epb_ctx* ctx, EighArgs& a) {
     EPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     allowed.fetch_or(bit);
   }
-  unsigned long long* counter = (unsigned long long*)(ctx->dstat + 28);
-  EPB_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), ctx->stream));
+  unsigned long long* counter = capturing(ctx) ? nullptr : (unsigned long long*)(ctx->dstat + 28);
+  EPB_TRY(scratch_begin(ctx));
+  if (counter) EPB_CUDA(cudaMemsetAsync(counter, 0, sizeof(*counter), ctx->stream));
   const int64_t blocks = std::min<int64_t>(a.batch, (int64_t)ctx->sm_count * std::max(1, 220 * 1024 / smem));
   prof_begin(ctx, EPB_PROF_EIGH);
   kern<<<(unsigned)blocks, NT, smem, ctx->stream>>>(a, counter);
   prof_end(ctx);
   EPB_LAUNCH_CHECK();
-  return EPB_OK;
+  return scratch_end(ctx);
 }
 
 // Dispatch on max order and precision. The mixed solver of orders 33..48 has its own instance: its shared

@@ -581,6 +581,7 @@ static int launch_big(epb_ctx* ctx, BigArgs a, int64_t batch) {
   const size_t slab_max = per_sm * sizeof(double2) * (size_t)ctx->sm_count;
   const size_t slab = (size_t)3 * NMAX * NMAX * sizeof(double2) * (size_t)grid;
   void* ws = nullptr;
+  EPB_TRY(scratch_begin(ctx));
   EPB_TRY(ws_get(ctx, EPB_WS_EIGH_BIG, (slab > slab_max ? slab : slab_max) + 256, &ws));
   a.scratch = (double2*)((uint8_t*)ws + 256);
   a.counter = (unsigned long long*)ws;
@@ -589,7 +590,7 @@ static int launch_big(epb_ctx* ctx, BigArgs a, int64_t batch) {
   eigh_big_kernel<NMAX, NT, MINB><<<(unsigned)grid, NT, SM::TOTAL, ctx->stream>>>(a);
   prof_end(ctx);
   EPB_LAUNCH_CHECK();
-  return EPB_OK;
+  return scratch_end(ctx);
 }
 
 // Launch the order-65..96 solver over a (uniform or varlen) batch; matrices of order <= n_lo are

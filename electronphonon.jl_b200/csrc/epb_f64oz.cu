@@ -584,6 +584,7 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
   const size_t ab = (size_t)(mt * KC * OZ_AB), bb = (size_t)(nt * KC * OZ_BB);
   const size_t sa = ((size_t)a.M * 4 + 255) / 256 * 256, sb = ((size_t)(nt * OZ_N) * 16 + 255) / 256 * 256;
   void* ws = nullptr;
+  EPB_TRY(scratch_begin(ctx));
   EPB_TRY(ws_try(ctx, EPB_WS_FOURIER, ab + bb + sa + sb, &ws));
   uint8_t* ap = (uint8_t*)ws;
   uint8_t* bp = ap + ab;
@@ -636,7 +637,8 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
     oz_gemm_kernel<<<(unsigned)std::min<int64_t>(ctx->sm_count, mt * tiles), OZ_THREADS, OZ_SMEM, ctx->stream>>>(g);
     EPB_LAUNCH_CHECK();
   }
-  return f64_gemm_guarded(ctx, a, mode, words, gen);
+  EPB_TRY(f64_gemm_guarded(ctx, a, mode, words, gen));
+  return scratch_end(ctx);
 }
 
 }  // namespace epb

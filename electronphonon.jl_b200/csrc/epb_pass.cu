@@ -278,7 +278,9 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
     pg.warm = false;
   }
   if (pg.exec) {
+    EPB_TRY(scratch_begin(ctx));
     EPB_CUDA(cudaGraphLaunch(pg.exec, ctx->stream));
+    EPB_TRY(scratch_end(ctx));
     ctx->launches += pg.launches;
   } else if (pg.warm) {
     cudaGraph_t graph = nullptr;
@@ -299,7 +301,9 @@ int epb_eph_pass(epb_ctx* ctx, epb_model* m, const double* xk, int64_t nk, const
     ce = cudaGraphInstantiate(&pg.exec, graph, 0);
     cudaGraphDestroy(graph);
     EPB_CUDA(ce);
+    EPB_TRY(scratch_begin(ctx));
     EPB_CUDA(cudaGraphLaunch(pg.exec, ctx->stream));
+    EPB_TRY(scratch_end(ctx));
     ctx->launches += pg.launches;
   } else {
     int st = eph_pass_run(ctx, m, xk, nk, xq, nq, prec, k_batch, sample_stride, ek_out, omega_out, g2sum_out, g2_sample,
