@@ -105,6 +105,8 @@ enum epb_prof_id {
   EPB_PROF_N
 };
 
+constexpr int EPB_DSTAT_OZ = 32;  // status words of the digit form (see epb_ctx::dstat)
+
 struct epb_prof_rec {
   cudaEvent_t a, b;
   int id;
@@ -124,8 +126,11 @@ struct epb_ctx {
   int fail_alloc_nth = 0;  // test hook
   // Small pinned host scratch for scalar read-backs.
   int64_t* pinned = nullptr;
-  // Device status words: [0] eigensolver non-convergence count, [1] eigensolver bad order count,
-  // [2] tensor-core GEMM timeout flag, [3] iq-hash miss count, [16] and [17] the digit form's words.
+  // Device status words (64): [0] eigensolver non-convergence count, [1] eigensolver bad order count,
+  // [2] tensor-core GEMM timeout flag, [3] iq-hash miss count, [4] slow-path count of the order-16 refinement,
+  // [5] MLP tensor-core timeout flag, [16..17] absolute maximum at model creation, [20..23] extents of an uneven
+  // batch and [24], [25] the counts of its tuning trials, [28..29] work counter of the FP64 Jacobi, [32..33] the digit
+  // form's words.
   int* dstat = nullptr;
   // instrumentation
   int64_t launches = 0;          // kernels launched by the library on this context
@@ -154,7 +159,6 @@ struct epb_ctx {
   // cuBLAS handle of the plain FP64 pass (its GEMMs are library ZGEMMs, as in the reference's GPU path),
   // created on first use
   void* cublas = nullptr;
-  int oz_gen = 0;  // products done in digit form (epb_f64oz.cu)
 };
 
 struct epb_rset {

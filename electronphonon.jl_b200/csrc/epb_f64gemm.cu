@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(T::THREADS, T::MINB) f64_gemm_kernel(F64GemmAr
 
 // The whole product in one wave, if words say that the digit form could not hold it (epb_f64oz.cu).
 template <class T, int MODE>
-__global__ void __launch_bounds__(T::THREADS, T::MINB) f64_gemm_guarded_kernel(F64GemmArgs a, const int* words, int gen) {
-  if (words[0] != gen && words[1] == 0) return;
+__global__ void __launch_bounds__(T::THREADS, T::MINB) f64_gemm_guarded_kernel(F64GemmArgs a, const int* words) {
+  if (words[0] == 0 && words[1] == 0) return;
   const int64_t mt = (a.M + T::BM - 1) / T::BM, nt = (a.N + T::BN - 1) / T::BN;
   for (int64_t t = blockIdx.x; t < mt * nt; t += gridDim.x) {
     gemm_tile<T, MODE>(a, t % mt * T::BM, t / mt * T::BN);
@@ -337,7 +337,7 @@ static int gemm_dispatch(epb_ctx* ctx, const F64GemmArgs& a) {
 }
 
 template <int MODE>
-static int launch_guarded(epb_ctx* ctx, const F64GemmArgs& a, const int* words, int gen) {
+static int launch_guarded(epb_ctx* ctx, const F64GemmArgs& a, const int* words) {
   using T = GemmTile<64, 64, 2, 4, 1, 8, 4, 2>;
   static std::atomic<uint64_t> allowed{0};
   const uint64_t bit = uint64_t(1) << (ctx->device & 63);
@@ -346,15 +346,15 @@ static int launch_guarded(epb_ctx* ctx, const F64GemmArgs& a, const int* words, 
     allowed.fetch_or(bit);
   }
   const size_t smem = T::smem(MODE == B_TABLE, a.K, a.L0 + a.L1 + a.L2);
-  f64_gemm_guarded_kernel<T, MODE><<<(unsigned)(2 * ctx->sm_count), T::THREADS, smem, ctx->stream>>>(a, words, gen);
+  f64_gemm_guarded_kernel<T, MODE><<<(unsigned)(2 * ctx->sm_count), T::THREADS, smem, ctx->stream>>>(a, words);
   EPB_LAUNCH_CHECK();
   return EPB_OK;
 }
 
-int f64_gemm_guarded(epb_ctx* ctx, const F64GemmArgs& a, int mode, const int* words, int gen) {
-  if (mode == B_MATRIX) return launch_guarded<B_MATRIX>(ctx, a, words, gen);
-  if (mode == B_TABLE) return launch_guarded<B_TABLE>(ctx, a, words, gen);
-  return launch_guarded<B_DIRECT>(ctx, a, words, gen);
+int f64_gemm_guarded(epb_ctx* ctx, const F64GemmArgs& a, int mode, const int* words) {
+  if (mode == B_MATRIX) return launch_guarded<B_MATRIX>(ctx, a, words);
+  if (mode == B_TABLE) return launch_guarded<B_TABLE>(ctx, a, words);
+  return launch_guarded<B_DIRECT>(ctx, a, words);
 }
 
 // The digit form where it pays and has its scratch, else the FP64 tensor cores.

@@ -28,6 +28,6 @@ struct F64GemmArgs {
 
 bool oz_pays(epb_ctx* ctx, const F64GemmArgs& a);
 int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode);
-int f64_gemm_guarded(epb_ctx* ctx, const F64GemmArgs& a, int mode, const int* words, int gen);
+int f64_gemm_guarded(epb_ctx* ctx, const F64GemmArgs& a, int mode, const int* words);
 
 }  // namespace epb

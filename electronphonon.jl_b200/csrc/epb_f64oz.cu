@@ -117,12 +117,10 @@ __device__ __forceinline__ OzRow oz_row(int64_t e, int tri_n) {
 
 // Shift of every complex row (largest of |re|, |im| over k); 8 rows x 32 k lanes per block.
 __global__ void __launch_bounds__(256) oz_row_shift_kernel(const double2* __restrict__ a, int64_t ld, int64_t M, int64_t K,
-                                                           int tri_n, int* __restrict__ shift, int* __restrict__ words,
-                                                           int gen) {
+                                                           int tri_n, int* __restrict__ shift, int* __restrict__ words) {
   __shared__ double red[32][9];
   const int r = threadIdx.x & 7, kl = threadIdx.x >> 3;
   const int64_t e = (int64_t)blockIdx.x * 8 + r;
-  if (blockIdx.x == 0 && threadIdx.x == 0) words[1] = 0;  // no wait of this product has run out yet
   double m = 0.0;
   bool bad = false;
   if (e < M) {
@@ -135,7 +133,7 @@ __global__ void __launch_bounds__(256) oz_row_shift_kernel(const double2* __rest
     }
   }
   red[kl][r] = m;
-  if (bad) words[0] = gen;
+  if (bad) words[0] = 1;
   __syncthreads();
   for (int o = 16; o > 0; o >>= 1) {
     if (kl < o) red[kl][r] = fmax(red[kl][r], red[kl + o][r]);
@@ -186,7 +184,7 @@ __global__ void __launch_bounds__(128) oz_pack_a_kernel(const double2* __restric
 template <bool TABLE>
 __global__ void __launch_bounds__(256) oz_pack_phase_kernel(const int4* __restrict__ rv, int64_t K, const double* __restrict__ xk,
                                                             int64_t N, int64_t KC, int lo0, int lo1, int lo2, int L0, int L1,
-                                                            int L2, uint8_t* __restrict__ out, int* __restrict__ words, int gen) {
+                                                            int L2, uint8_t* __restrict__ out, int* __restrict__ words) {
   extern __shared__ __align__(16) unsigned char oz_sm[];
   double2* tab = reinterpret_cast<double2*>(oz_sm);  // [L0 + L1 + L2][128]
   const int h = threadIdx.x & 1, j = threadIdx.x >> 1;  // half of a chunk, point
@@ -230,13 +228,13 @@ __global__ void __launch_bounds__(256) oz_pack_phase_kernel(const int4* __restri
     }
     oz_store<OZ_PLANE>(out + ((int64_t)blockIdx.x * KC + c) * OZ_BB, j, h, v);
   }
-  if (bad) words[0] = gen;
+  if (bad) words[0] = 1;
 }
 
 // Columns of a K x N matrix: one warp per column finds its shift and packs it.
 __global__ void __launch_bounds__(128) oz_pack_b_kernel(const double2* __restrict__ b, int64_t ldb, int64_t K, int64_t N,
                                                         int64_t KC, double2* __restrict__ unscale, uint8_t* __restrict__ out,
-                                                        int* __restrict__ words, int gen) {
+                                                        int* __restrict__ words) {
   const int lane = threadIdx.x & 31;
   const int64_t col = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (col >= N) return;
@@ -249,7 +247,7 @@ __global__ void __launch_bounds__(128) oz_pack_b_kernel(const double2* __restric
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (bad) words[0] = gen;
+  if (bad) words[0] = 1;
   const int e = oz_shift(m);
   const double2 sc = oz_scale(e);
   if (lane == 0) unscale[col] = oz_scale(-e);
@@ -590,8 +588,8 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
   uint8_t* bp = ap + ab;
   int* ash = (int*)(bp + bb);
   double2* bsc = (double2*)((char*)ash + sa);
-  int* words = ctx->dstat + 16;  // [0] generation of the last product with an operand outside the digits, [1] a wait ran out
-  const int gen = ++ctx->oz_gen;
+  int* words = ctx->dstat + EPB_DSTAT_OZ;  // [0] an operand is outside the digits, [1] a wait ran out
+  EPB_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(int), ctx->stream));
   static std::atomic<uint64_t> allowed{0};
   const uint64_t bit = uint64_t(1) << (ctx->device & 63);
   if (!(allowed.load() & bit)) {
@@ -599,7 +597,7 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
     EPB_CUDA(cudaFuncSetAttribute(oz_pack_phase_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     allowed.fetch_or(bit);
   }
-  oz_row_shift_kernel<<<(unsigned)cdiv(a.M, 8), 256, 0, ctx->stream>>>(a.A, a.lda, a.M, a.K, a.tri_n, ash, words, gen);
+  oz_row_shift_kernel<<<(unsigned)cdiv(a.M, 8), 256, 0, ctx->stream>>>(a.A, a.lda, a.M, a.K, a.tri_n, ash, words);
   EPB_LAUNCH_CHECK();
   oz_pack_a_kernel<<<dim3((unsigned)cdiv(a.M, 64), (unsigned)KC), 128, 0, ctx->stream>>>(a.A, a.lda, a.M, a.K, KC, a.tri_n,
                                                                                         ash, ap);
@@ -607,16 +605,16 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
   for (int64_t t0 = 0; t0 * OZ_N < a.N; t0 += nt) {
     const int64_t c0 = t0 * OZ_N, n = std::min(nt * OZ_N, a.N - c0), tiles = cdiv(n, OZ_N);
     if (mode == B_MATRIX) {
-      oz_pack_b_kernel<<<(unsigned)cdiv(n, 4), 128, 0, ctx->stream>>>(a.B + c0 * a.ldb, a.ldb, a.K, n, KC, bsc, bp, words, gen);
+      oz_pack_b_kernel<<<(unsigned)cdiv(n, 4), 128, 0, ctx->stream>>>(a.B + c0 * a.ldb, a.ldb, a.K, n, KC, bsc, bp, words);
     } else {
       const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>(KC, 6 * ctx->sm_count / tiles));
       const dim3 grid((unsigned)tiles, gy);
       if (mode == B_TABLE)
         oz_pack_phase_kernel<true><<<grid, 256, sizeof(double2) * OZ_N * (a.L0 + a.L1 + a.L2), ctx->stream>>>(
-            a.rv, a.K, a.xk + 3 * c0, n, KC, a.lo0, a.lo1, a.lo2, a.L0, a.L1, a.L2, bp, words, gen);
+            a.rv, a.K, a.xk + 3 * c0, n, KC, a.lo0, a.lo1, a.lo2, a.L0, a.L1, a.L2, bp, words);
       else
         oz_pack_phase_kernel<false><<<grid, 256, 0, ctx->stream>>>(a.rv, a.K, a.xk + 3 * c0, n, KC, 0, 0, 0, 0, 0, 0, bp,
-                                                                   words, gen);
+                                                                   words);
     }
     EPB_LAUNCH_CHECK();
     OzGemmArgs g;
@@ -637,7 +635,7 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
     oz_gemm_kernel<<<(unsigned)std::min<int64_t>(ctx->sm_count, mt * tiles), OZ_THREADS, OZ_SMEM, ctx->stream>>>(g);
     EPB_LAUNCH_CHECK();
   }
-  EPB_TRY(f64_gemm_guarded(ctx, a, mode, words, gen));
+  EPB_TRY(f64_gemm_guarded(ctx, a, mode, words));
   return scratch_end(ctx);
 }
 

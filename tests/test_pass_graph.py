@@ -127,3 +127,30 @@ def test_sum_in_a_callers_graph(graph_mode):
         g.replay()
         assert (out - eager).abs().max().item() <= bar
     del g
+
+
+@pytest.mark.gpu
+def test_not_finite_once(graph_mode):
+    """A replay whose points are NaN is done by the FP64 tensor cores; the next one, finite again, has the bits of the
+    digit form."""
+    import torch
+
+    from epb200 import pipeline as P
+    from epb200.batched import jl
+
+    dm = P.DeviceModel(synth.config2_model(seed=5, n_el=1, n_ph=2, nw=16, natom=4))
+    xk, xq = jl(synth.random_kpoints(2, 40)), jl(synth.random_kpoints(4096, 41))
+    out = None
+    for _ in range(3):  # eager, capture, replay
+        out = _run(P, dm, xk, xq, out, k_batch=2)
+    ref = _arrays(out)
+    q = xq.clone()
+    xq[5] = np.nan
+    out = _run(P, dm, xk, xq, out, k_batch=2)
+    assert np.isnan(_arrays(out)[1][:, 5]).any()
+    xq.copy_(q)
+    for _ in range(2):
+        out = _run(P, dm, xk, xq, out, k_batch=2)
+        for a, b in zip(_arrays(out), ref):
+            np.testing.assert_array_equal(a, b)
+    dm.close()
