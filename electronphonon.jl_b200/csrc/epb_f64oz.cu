@@ -61,6 +61,7 @@ constexpr int OZ_SMEM = OZ_STAGES * OZ_STAGE + 1024 + 256;
 constexpr int OZ_BUF = 4;                      // accumulator buffers of OZ_N TMEM columns
 constexpr int OZ_EPI0 = 4, OZ_EPIW = 16;       // epilogue warps
 constexpr int OZ_THREADS = 32 * (OZ_EPI0 + OZ_EPIW);
+constexpr int64_t OZ_RUN = 512 << 20;          // bytes of A's planes at a time (B: half)
 constexpr int64_t OZ_K_MAX = 4000;             // 7 * 2 K 2^14 < 2^31
 
 // Largest e with |x| 2^e within seven balanced digits (127.498 * 256^6) for |x| <= m.
@@ -572,15 +573,43 @@ bool oz_pays(epb_ctx* ctx, const F64GemmArgs& a) {
   return oz < 0.9 * dm;
 }
 
-// C = A B by digits, or EPB_ERR_UNSUPPORTED when there is no scratch for them. phase: B is the phase of a.xk.
+// Planes of the n columns from c0 (a whole number of tiles from the first).
+static int oz_pack_b(epb_ctx* ctx, const F64GemmArgs& a, int mode, int64_t c0, int64_t n, int64_t KC, double2* scale,
+                     uint8_t* out, int* words) {
+  if (mode == B_MATRIX) {
+    oz_pack_b_kernel<<<(unsigned)cdiv(n, 4), 128, 0, ctx->stream>>>(a.B + c0 * a.ldb, a.ldb, a.K, n, KC, scale, out, words);
+  } else {
+    const int64_t tiles = cdiv(n, OZ_N);
+    const dim3 grid((unsigned)tiles, (unsigned)std::max<int64_t>(1, std::min<int64_t>(KC, 6 * ctx->sm_count / tiles)));
+    if (mode == B_TABLE)
+      oz_pack_phase_kernel<true><<<grid, 256, sizeof(double2) * OZ_N * (a.L0 + a.L1 + a.L2), ctx->stream>>>(
+          a.rv, a.K, a.xk + 3 * c0, n, KC, a.lo0, a.lo1, a.lo2, a.L0, a.L1, a.L2, out, words);
+    else
+      oz_pack_phase_kernel<false><<<grid, 256, 0, ctx->stream>>>(a.rv, a.K, a.xk + 3 * c0, n, KC, 0, 0, 0, 0, 0, 0, out, words);
+  }
+  EPB_LAUNCH_CHECK();
+  return EPB_OK;
+}
+
+// C = A B by digits, or EPB_ERR_UNSUPPORTED when there is no scratch for them. A is packed in runs of at most OZ_RUN
+// bytes, B of half that: all planes of a g(Re, Rp) of 384000 rows and 729 R would take 8 GB of a workspace that lives as
+// long as the context, where runs of whole waves of tiles take 0.5 GB (96 k of it, rotation to 4 bands included: 5.57 ms
+// in one run, 5.90 ms in 21; in runs of 256 MB that are no whole waves 6.88). The B runs of several A runs are packed again
+// for each, which is under a hundredth of the run's MMAs. The rows of a triangle do not split by tiles; there all of A is
+// packed at once, up to two runs.
 int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
   const int64_t rows = a.tri_n ? (int64_t)a.tri_n * a.tri_n : 2 * a.M;
-  const int64_t mt = cdiv(rows, OZ_M), KC = cdiv(2 * a.K, OZ_KC);
-  // columns per run: whole waves of tiles, B planes of at most 256 MB
-  int64_t nt = std::min<int64_t>(cdiv(a.N, OZ_N), std::max<int64_t>(1, ((int64_t)256 << 20) / (KC * OZ_BB)));
-  if (nt < cdiv(a.N, OZ_N) && nt * mt > ctx->sm_count) nt = std::max<int64_t>(1, nt * mt / ctx->sm_count * ctx->sm_count / mt);
+  const int64_t all_mt = cdiv(rows, OZ_M), all_nt = cdiv(a.N, OZ_N), KC = cdiv(2 * a.K, OZ_KC);
+  const int64_t cap = std::max<int64_t>(1, OZ_RUN / (KC * OZ_AB));
+  if (a.tri_n && all_mt > 2 * cap) return EPB_ERR_UNSUPPORTED;
+  int64_t mt = a.tri_n ? all_mt : std::min(all_mt, cap), nt = std::min(all_nt, std::max<int64_t>(1, cap / 2));
+  // runs of whole waves of tiles
+  const int64_t sm = ctx->sm_count;
+  if (mt < all_mt && nt * mt > sm) mt = std::max<int64_t>(1, nt * mt / sm * sm / nt);
+  if (nt < all_nt && nt * mt > sm) nt = std::max<int64_t>(1, nt * mt / sm * sm / mt);
   const size_t ab = (size_t)(mt * KC * OZ_AB), bb = (size_t)(nt * KC * OZ_BB);
-  const size_t sa = ((size_t)a.M * 4 + 255) / 256 * 256, sb = ((size_t)(nt * OZ_N) * 16 + 255) / 256 * 256;
+  const int64_t mc = a.tri_n ? a.M : mt * (OZ_M / 2);  // complex rows per run
+  const size_t sa = ((size_t)mc * 4 + 255) / 256 * 256, sb = ((size_t)(nt * OZ_N) * 16 + 255) / 256 * 256;
   void* ws = nullptr;
   EPB_TRY(scratch_begin(ctx));
   EPB_TRY(ws_try(ctx, EPB_WS_FOURIER, ab + bb + sa + sb, &ws));
@@ -597,43 +626,34 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
     EPB_CUDA(cudaFuncSetAttribute(oz_pack_phase_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     allowed.fetch_or(bit);
   }
-  oz_row_shift_kernel<<<(unsigned)cdiv(a.M, 8), 256, 0, ctx->stream>>>(a.A, a.lda, a.M, a.K, a.tri_n, ash, words);
-  EPB_LAUNCH_CHECK();
-  oz_pack_a_kernel<<<dim3((unsigned)cdiv(a.M, 64), (unsigned)KC), 128, 0, ctx->stream>>>(a.A, a.lda, a.M, a.K, KC, a.tri_n,
-                                                                                        ash, ap);
-  EPB_LAUNCH_CHECK();
-  for (int64_t t0 = 0; t0 * OZ_N < a.N; t0 += nt) {
-    const int64_t c0 = t0 * OZ_N, n = std::min(nt * OZ_N, a.N - c0), tiles = cdiv(n, OZ_N);
-    if (mode == B_MATRIX) {
-      oz_pack_b_kernel<<<(unsigned)cdiv(n, 4), 128, 0, ctx->stream>>>(a.B + c0 * a.ldb, a.ldb, a.K, n, KC, bsc, bp, words);
-    } else {
-      const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>(KC, 6 * ctx->sm_count / tiles));
-      const dim3 grid((unsigned)tiles, gy);
-      if (mode == B_TABLE)
-        oz_pack_phase_kernel<true><<<grid, 256, sizeof(double2) * OZ_N * (a.L0 + a.L1 + a.L2), ctx->stream>>>(
-            a.rv, a.K, a.xk + 3 * c0, n, KC, a.lo0, a.lo1, a.lo2, a.L0, a.L1, a.L2, bp, words);
-      else
-        oz_pack_phase_kernel<false><<<grid, 256, 0, ctx->stream>>>(a.rv, a.K, a.xk + 3 * c0, n, KC, 0, 0, 0, 0, 0, 0, bp,
-                                                                   words);
+  for (int64_t r0 = 0; r0 < a.M; r0 += mc) {
+    const int64_t m = std::min(mc, a.M - r0), mrows = a.tri_n ? rows : 2 * m;
+    const double2* A = a.A + r0;
+    oz_row_shift_kernel<<<(unsigned)cdiv(m, 8), 256, 0, ctx->stream>>>(A, a.lda, m, a.K, a.tri_n, ash, words);
+    EPB_LAUNCH_CHECK();
+    oz_pack_a_kernel<<<dim3((unsigned)cdiv(m, 64), (unsigned)KC), 128, 0, ctx->stream>>>(A, a.lda, m, a.K, KC, a.tri_n, ash, ap);
+    EPB_LAUNCH_CHECK();
+    for (int64_t t0 = 0; t0 < all_nt; t0 += nt) {
+      const int64_t c0 = t0 * OZ_N, n = std::min(nt * OZ_N, a.N - c0), tiles = cdiv(n, OZ_N);
+      if (r0 == 0 || nt < all_nt) EPB_TRY(oz_pack_b(ctx, a, mode, c0, n, KC, bsc, bp, words));
+      OzGemmArgs g;
+      g.A = ap;
+      g.B = bp;
+      g.KC = (int)KC;
+      g.m_tiles = cdiv(mrows, OZ_M);
+      g.n_tiles = tiles;
+      g.rows = mrows;
+      g.cols = n;
+      g.a_shift = ash;
+      g.b_scale = mode == B_MATRIX ? bsc : nullptr;
+      g.C = (double*)(a.C + r0 + c0 * a.ldc);
+      g.ldc2 = 2 * a.ldc;
+      g.tri_n = a.tri_n;
+      g.err = words + 1;
+      g.timeout = 4000000000LL;  // ~2 s
+      oz_gemm_kernel<<<(unsigned)std::min<int64_t>(ctx->sm_count, g.m_tiles * tiles), OZ_THREADS, OZ_SMEM, ctx->stream>>>(g);
+      EPB_LAUNCH_CHECK();
     }
-    EPB_LAUNCH_CHECK();
-    OzGemmArgs g;
-    g.A = ap;
-    g.B = bp;
-    g.KC = (int)KC;
-    g.m_tiles = mt;
-    g.n_tiles = tiles;
-    g.rows = rows;
-    g.cols = n;
-    g.a_shift = ash;
-    g.b_scale = mode == B_MATRIX ? bsc : nullptr;
-    g.C = (double*)(a.C + c0 * a.ldc);
-    g.ldc2 = 2 * a.ldc;
-    g.tri_n = a.tri_n;
-    g.err = words + 1;
-    g.timeout = 4000000000LL;  // ~2 s
-    oz_gemm_kernel<<<(unsigned)std::min<int64_t>(ctx->sm_count, mt * tiles), OZ_THREADS, OZ_SMEM, ctx->stream>>>(g);
-    EPB_LAUNCH_CHECK();
   }
   EPB_TRY(f64_gemm_guarded(ctx, a, mode, words));
   return scratch_end(ctx);
