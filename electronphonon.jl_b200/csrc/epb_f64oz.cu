@@ -4,11 +4,13 @@
 // per row (A) or column (B) by a power of two to a 55-bit integer and written in seven balanced base-256 digits,
 //   x 2^e = sum_i d_i 256^(6-i),   d_i in [-128, 127],
 // each an int8 operand plane. C = sum_{i+j <= 6} 2^(8 (12-i-j)) D_i E_j: 28 int8 GEMMs whose int32 accumulators
-// are exact (7 K' 2^14 < 2^31), one accumulator per i + j. The pairs left out are below 2^-55 of the scaled
-// operands; the seven sums are joined in 64-bit integers and one FP64 FMA. Only the operands and the final sum are
-// rounded, so the error against extended precision is under half that of the FP64 FMA chain (Gaussian rows
-// decaying as exp(-|R| / 1.5), normwise, on the device: 125 R 2.8e-16 against 5.3e-16, 343 R 4.2e-16 / 8.7e-16,
-// 729 R 5.8e-16 / 1.27e-15).
+// are exact (7 K' 2^14 < 2^31), one accumulator per i + j. The seven sums are joined in 64-bit integers and one FP64 FMA.
+// What is lost, per real product and in units of the row's largest |a| times the column's largest |b|: the pairs left
+// out, six products of digits of weight 2^40 against 2^108 at least, so up to 2^-51.4 and 2^-54.3 in rms; and the
+// operands' own rounding, 2^-55 each. That is on the scale of the rounding of an FP64 FMA onto a sum of that size, and
+// unlike it does not grow with the partial sums. Gaussian rows decaying as exp(-|R| / 1.5), error against extended
+// precision, normwise, on the device: 125 R 2.8e-16 against 5.3e-16 for the FMA chain, 343 R 4.2e-16 / 8.7e-16, 729 R
+// 5.8e-16 / 1.27e-15.
 //
 // Measured against the FP64 tensor cores at 85 % of their peak, packing included: 3072 x 125 x 8192 0.88 -> 0.34 ms
 // (cuBLAS ZGEMM 0.78), x 729 1.36 ms (108 TFLOP/s of FP64 work); upper triangles of 32-band H at 98292 points, 1331 R
@@ -32,13 +34,15 @@
 // issuing thread's own instructions and waits 60. The accumulators of consecutive passes rotate through four TMEM
 // buffers, so that MMAs start in a free one while the others are read out.
 //
-// Anything the digits cannot hold (an infinity or NaN in an operand) raises a device word, and so does a wait that
-// ran out; the FP64 tensor-core kernel then does the product again (f64_gemm_guarded), so results are those of
-// that kernel. Without enough scratch the caller uses it in the first place.
+// Anything the digits cannot hold (an infinity or NaN in an operand, a column of a matrix B that is far from flat, see
+// oz_pack_b_kernel) raises a device word, and so does a wait that ran out; the FP64 tensor-core kernel then does the
+// product (f64_gemm_guarded), so results are those of that kernel. Without enough scratch the caller uses it in the
+// first place.
 #include <algorithm>
 #include <atomic>
 #include <climits>
 #include <cmath>
+#include <math_constants.h>
 
 #include "epb_f64gemm.cuh"
 #include "epb_umma.cuh"
@@ -232,7 +236,11 @@ __global__ void __launch_bounds__(256) oz_pack_phase_kernel(const int4* __restri
   if (bad) words[0] = 1;
 }
 
-// Columns of a K x N matrix: one warp per column finds its shift and packs it.
+// Columns of a K x N matrix: one warp per column finds its shift and packs it. Digits hold every entry to the same
+// absolute step, so a column must be as flat as a phase, every entry at least half the largest: then
+// sum |a_k| |b_k| >= max |a| max |b| / 2 whatever the row, and an error on the scale of the maxima is one on the scale of
+// the terms. A graded column against a graded row could have its largest products where neither is large; it raises the
+// word, as an infinity does.
 __global__ void __launch_bounds__(128) oz_pack_b_kernel(const double2* __restrict__ b, int64_t ldb, int64_t K, int64_t N,
                                                         int64_t KC, double2* __restrict__ unscale, uint8_t* __restrict__ out,
                                                         int* __restrict__ words) {
@@ -240,15 +248,20 @@ __global__ void __launch_bounds__(128) oz_pack_b_kernel(const double2* __restric
   const int64_t col = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (col >= N) return;
   const double2* p = b + col * ldb;
-  double m = 0.0;
+  double m = 0.0, least = CUDART_INF;
   bool bad = false;
   for (int64_t k = lane; k < K; k += 32) {
     const double2 v = p[k];
     bad |= !(isfinite(v.x) && isfinite(v.y));
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+    const double big = fmax(fabs(v.x), fabs(v.y));
+    m = fmax(m, big);
+    least = fmin(least, big);
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (bad) words[0] = 1;
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
+  }
+  if (bad || least < 0.5 * m) words[0] = 1;
   const int e = oz_shift(m);
   const double2 sc = oz_scale(e);
   if (lane == 0) unscale[col] = oz_scale(-e);
@@ -277,6 +290,7 @@ struct OzGemmArgs {
   double* C;              // complex matrix as doubles
   int64_t ldc2;           // doubles between columns
   int tri_n;
+  const int* outside;     // an operand is outside the digits: nothing to do
   int* err;
   long long timeout;
 };
@@ -301,6 +315,7 @@ __device__ __forceinline__ double oz_double(uint32_t x) {
 }
 
 __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(OzGemmArgs a) {
+  if (*a.outside) return;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -482,7 +497,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(OzGemmArgs a) {
     uint32_t acc = 0;
     for (int64_t t = blockIdx.x; t < total; t += gridDim.x, acc += OZ_PL) {
       const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + part * 32;
-      // Digit sums 4, 5, 6, 3, 2 join exactly in 64-bit integers (below 2^60, in units of 2^48), one wide multiply-add
+      // Digit sums 4, 5, 6, 3, 2 join exactly in 64-bit integers (below 2^61, in units of 2^48), one wide multiply-add
       // each, so that a buffer goes back to the MMAs soon; that integer rounds once to FP64 and the last two sums add
       // to it by FMA.
       long long v[32];
@@ -649,6 +664,7 @@ int oz_gemm(epb_ctx* ctx, const F64GemmArgs& a, int mode) {
       g.C = (double*)(a.C + r0 + c0 * a.ldc);
       g.ldc2 = 2 * a.ldc;
       g.tri_n = a.tri_n;
+      g.outside = words;
       g.err = words + 1;
       g.timeout = 4000000000LL;  // ~2 s
       oz_gemm_kernel<<<(unsigned)std::min<int64_t>(ctx->sm_count, g.m_tiles * tiles), OZ_THREADS, OZ_SMEM, ctx->stream>>>(g);
