@@ -185,7 +185,7 @@ static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
 }
 
 bool rot64_covers(int nw, int nm);
-bool rot64_pays(int nw, int nbk, int nbkq, int nm);
+bool rot64_pays(epb_ctx* ctx, int nw, int nbk, int nbkq, int nm, int64_t nq);
 int eph_rot64(epb_ctx* ctx, const double2* g, int64_t ldg, int nw, int nbk, int nm, int64_t nq, const double2* ukq,
               int nbkq, const double2* uph, const double* omega, double2* ep, double* g2);
 int eph_rot64(epb_ctx* ctx, const float2* g, int64_t ldg, int nw, int nbk, int nm, int64_t nq, const double2* ukq,
@@ -200,7 +200,7 @@ static int eph_rotations_t(epb_ctx* ctx, const G* g, int64_t ldg, int nw, int nb
   EPB_CHECK_ARG(smem <= 200 * 1024, "eph rotations: block (nw=%d, nbk=%d, nm=%d) exceeds shared memory",
                 nw, nbk, nm);
   const size_t ng = sizeof(G) * (size_t)ldg * nq, no = (size_t)nbkq * nbk * nm * nq;
-  if (rot64_covers(nw, nm) && rot64_pays(nw, nbk, nbkq, nm) && !overlap(g, ng, ep, sizeof(double2) * no) &&
+  if (rot64_covers(nw, nm) && rot64_pays(ctx, nw, nbk, nbkq, nm, nq) && !overlap(g, ng, ep, sizeof(double2) * no) &&
       !overlap(g, ng, g2, sizeof(double) * no))
     return eph_rot64(ctx, g, ldg, nw, nbk, nm, nq, ukq, nbkq, uph, omega, ep, g2);
   static bool attr = false;

@@ -16,6 +16,7 @@
 // per k, now 0.29. The next mode's g is fetched during this one's DMMAs (without that 0.39 / 0.50 ms).
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "epb_common.cuh"
 
@@ -375,14 +376,35 @@ static int r64_orders(epb_ctx* ctx, const G* g, const Rot64Args& a) {
 // Whether the register kernel covers a shape: all T of a lane (4 nm doubles) and its part of u_kq stay in
 // registers up to 15 modes and 32 bands. Beyond, the shared-memory kernel (or the library GEMMs of the pass).
 bool rot64_covers(int nw, int nm) { return nw <= 32 && nm <= 15; }
-// Whether it is also the faster one: a band slice of a few bands leaves most of an 8 x 8 tile empty, and the
-// shared-memory kernel works on live outputs only. Nanoseconds per q and SM of both, fitted to (bands k+q x k, modes;
-// measured register / shared memory, us for all q): 16 x 16, 12, 8192 q 273 / 2010; 16 x 2 183 / 240; 3 x 6, 4109 q
-// 47 / 43; 4 x 3, 6420 q 62 / 27; 10 x 3, 9 modes, 6428 q 76 / 48; 1 x 1, 8192 q 82 / 25; 2 x 2, 3 modes 20 / 21.
-bool rot64_pays(int nw, int nbk, int nbkq, int nm) {
-  const double tiles = ((nbkq + 7) / 8) * ((nbk + 7) / 8);
-  const double reg = tiles * (100.0 + 8.0 * nm * nm + 6.0 * ((nw + 3) / 4) * nm);
-  return reg <= std::max(450.0, 0.3 * nbkq * nbk * nm * (nw + nm));
+// Whether it is also the faster one: a band slice of a few bands leaves most of an 8 x 8 tile empty, a short q list leaves
+// most warps without an item, and one warp does all modes of an item in a chain; the shared-memory kernel works on live
+// outputs only, a block per q. Microseconds of the three kernels (launch, rounds of blocks or warps that do not fit the
+// chip at once, chains within a round, work per SM), fitted to 900 random shapes of 1 to 32 bands, 1 to 15 modes and 30
+// to 9000 q that were timed both ways: 21 % off in rms for shared memory, 11 % for the others. A tenth in favour of shared
+// memory leaves the fewest shapes slower than it (on 900 other shapes 17 by more than 5 %). Where the line lies (bands k+q
+// x k, of bands, modes, q: shared memory / registers, us): 5 x 3 of 17, 9, 4000 22.6 / 54.4; 8 x 8 of 8, 15, 100
+// 12.3 / 18.5; 6 x 6 of 6, 15, 4000 51 / 72; 16 x 2 of 16, 12, 8192 240 / 183; 16 x 16 of 16, 12, 8192 2010 / 273.
+bool rot64_pays(epb_ctx* ctx, int nw, int nbk, int nbkq, int nm, int64_t nq) {
+  const double sm = ctx->sm_count, q = (double)nq;
+  const int tiles = ((nbkq + 7) / 8) * ((nbk + 7) / 8), slot = (nm - 1) / 3;  // which of the mode counts 3, 6, .. 15
+  const double ks = nw <= 16 ? (nw + 3) / 4 : 8, mk = nm * ks, m2 = nm * nm;
+  // shared memory: blocks per SM by threads and memory; elements of T per thread
+  const int64_t nt = (int64_t)nbkq * nbk * nm, ng = (int64_t)nw * nbk * nm;
+  const double fit = std::floor(227.0 * 1024 / (16.0 * (ng + nt + (int64_t)nw * nbkq + nm * nm) + 1024));
+  const double blocks = std::min(8.0, std::max(1.0, fit)), ro = std::ceil(q / (sm * blocks)), et = std::ceil(nt / 256.0);
+  const double shared = 7.86 + ro * (0.0495 + et * (0.0604 * nw + 0.0048 * nm)) + 0.000141 * q / sm * nt * (nw + nm);
+  double reg;
+  const size_t stage = (size_t)R64Stage<double2>(nw, nbk, nm, nbkq).total * 16;
+  if (tiles >= R64_WARPS && stage <= R64_STAGE_MAX) {
+    const double per = std::min(nm > 9 ? 2.0 : nm > 3 ? 3.0 : 4.0, std::floor(227.0 * 1024 / (2.0 * stage + 2048)));
+    const double rs = std::ceil(q / (sm * per)), e = (tiles + R64_WARPS - 1) / R64_WARPS;
+    reg = 6.35 + rs * (0.527 + e * (0.0214 * mk + 0.0171 * m2)) + q / sm * (tiles * (0.00767 * mk + 0.00235 * m2) + 6.32e-6 * stage);
+  } else {
+    static const int per_lo[] = {6, 4, 4, 3, 2}, per_hi[] = {3, 3, 2, 2, 2};  // blocks per SM by registers
+    const double rd = std::ceil(q * tiles / (sm * R64_WARPS * (nw > 16 ? per_hi : per_lo)[slot]));
+    reg = 6.44 + rd * (0.447 + 0.0319 * mk + 0.0362 * m2) + q / sm * tiles * (0.00935 * mk + 0.00185 * m2);
+  }
+  return reg <= 0.9 * shared;
 }
 
 int eph_rot64(epb_ctx* ctx, const double2* g, int64_t ldg, int nw, int nbk, int nm, int64_t nq, const double2* ukq,
