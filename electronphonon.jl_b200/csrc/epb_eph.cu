@@ -178,7 +178,7 @@ __global__ void eph_rot_kernel(const G* __restrict__ g, int64_t ldg, const doubl
   }
 }
 
-// Two buffers share memory (a caller that writes ep over g keeps the kernel that reads a whole block first).
+// Two buffers share memory (a caller that writes over an input keeps the kernel that reads all of a q first).
 static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
   const char *x = (const char*)a, *y = (const char*)b;
   return x && y && x < y + nb && y < x + na;
@@ -199,9 +199,11 @@ static int eph_rotations_t(epb_ctx* ctx, const G* g, int64_t ldg, int nw, int nb
   size_t smem = sizeof(double2) * ((size_t)nw * nbk * nm + (size_t)nbkq * nbk * nm + nw * nbkq + nm * nm);
   EPB_CHECK_ARG(smem <= 200 * 1024, "eph rotations: block (nw=%d, nbk=%d, nm=%d) exceeds shared memory",
                 nw, nbk, nm);
-  const size_t ng = sizeof(G) * (size_t)ldg * nq, no = (size_t)nbkq * nbk * nm * nq;
-  if (rot64_covers(nw, nm) && rot64_pays(ctx, nw, nbk, nbkq, nm, nq) && !overlap(g, ng, ep, sizeof(double2) * no) &&
-      !overlap(g, ng, g2, sizeof(double) * no))
+  const size_t no = (size_t)nbkq * nbk * nm * nq;
+  auto over = [&](const void* in, size_t n) { return overlap(in, n, ep, sizeof(double2) * no) || overlap(in, n, g2, sizeof(double) * no); };
+  const bool in_place = over(g, sizeof(G) * (size_t)ldg * nq) || over(ukq, sizeof(double2) * (size_t)nw * nbkq * nq) ||
+                        over(uph, sizeof(double2) * (size_t)nm * nm * nq) || over(omega, sizeof(double) * (size_t)nm * nq);
+  if (!in_place && rot64_covers(nw, nm) && rot64_pays(ctx, nw, nbk, nbkq, nm, nq))
     return eph_rot64(ctx, g, ldg, nw, nbk, nm, nq, ukq, nbkq, uph, omega, ep, g2);
   static bool attr = false;
   if (!attr) {

@@ -48,3 +48,26 @@ def test_lists(nw, nbk, nbkq, nm, nq):
     only = torch.full_like(g2, 7.0)
     B.eph_apply_rotations(None, dg, du, dp, g2_out=only[:nq], omega=dw)
     assert torch.equal(only, g2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("over", ["g", "ukq", "uph"])
+def test_over_an_input(over):
+    """ep written over an input whose blocks of a q are as large as its own: every q is read before it is written."""
+    import torch
+
+    from epb200 import batched as B
+
+    nw, nbk, nbkq, nm, nq = {"g": (10, 5, 10, 6, 2000), "ukq": (16, 4, 16, 4, 6000), "uph": (9, 1, 9, 9, 3000)}[over]
+    rng = np.random.default_rng(nq)
+
+    def cn(*s):
+        return B.jl(np.asfortranarray(rng.standard_normal(s) + 1j * rng.standard_normal(s)))
+
+    args = {"g": cn(nw, nbk, nm, nq), "ukq": cn(nw, nbkq, nq), "uph": cn(nm, nm, nq)}
+    g, u, p = (B.host(args[k]).copy() for k in ("g", "ukq", "uph"))
+    ref = _rotate(g, u.conj(), p)
+    bar = (nw + nm + 16) * EPS * _rotate(np.abs(g), np.abs(u), np.abs(p))
+    ep = args[over].view(nq, nm, nbk, nbkq)
+    B.eph_apply_rotations(ep, args["g"], args["ukq"], args["uph"])
+    assert (np.abs(B.host(ep) - ref) <= bar).all()
