@@ -111,11 +111,11 @@ __device__ __forceinline__ int sturm_count(const T* d, const T* e2, int n, T sig
 // step after the last: the next column follows from u and w before the block update, so the sum over its lanes
 // runs between the update's FMAs instead of at the head of the next step.
 template <typename T, int N, int J0>
-__device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSmem<T, N>& s, int lane, T& dk, T& ek2,
-                                                  T& xn2, T& xr, T& xi) {
+__device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSmem<T, N>& s, int lane, int n, T& dk,
+                                                  T& ek2, T& xn2, T& xr, T& xi) {
   constexpr int KEND = (J0 + 8 < N - 1) ? J0 + 8 : N - 1;
 #pragma unroll 1
-  for (int k = J0; k < KEND; ++k) {
+  for (int k = J0; k < KEND && k < n; ++k) {  // the columns of the padding are zero
     // (xr, xi): column k, row `lane`; column k + 1 is picked for its early update
     T nr = 0, ni = 0;
 #pragma unroll
@@ -127,7 +127,7 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
       dk = xr;
       ek2 = xn2;
     }
-    if (k == N - 2) break;      // last off-diagonal: no reflection left to apply
+    if (k == N - 2 || k == n - 1) break;  // last off-diagonal, or last row of the matrix: no reflection left to apply
     const T x1r = __shfl_sync(0xffffffffu, xr, k + 1, N), x1i = __shfl_sync(0xffffffffu, xi, k + 1, N);
     const T a2 = x1r * x1r + x1i * x1i;
     T rx, ra;
@@ -209,15 +209,15 @@ __device__ __forceinline__ void householder_phase(T (&ar)[N], T (&ai)[N], TriSme
 
 // Reduce the matrix held row-wise in (ar, ai) to tridiagonal form; writes d, e2 to shared memory.
 template <typename T, int N>
-__device__ __forceinline__ void householder_tridiag(T (&ar)[N], T (&ai)[N], TriSmem<T, N>& s, int lane) {
+__device__ __forceinline__ void householder_tridiag(T (&ar)[N], T (&ai)[N], TriSmem<T, N>& s, int lane, int n) {
   static_assert(N == 8 || N == 16 || N == 32, "the reduction is laid out in phases of eight steps");
   T dk = 0, ek2 = 0, xn2 = group_sum<N>(lane > 0 ? ar[0] * ar[0] + ai[0] * ai[0] : T(0));
   T xr = ar[0], xi = ai[0];
-  householder_phase<T, N, 0>(ar, ai, s, lane, dk, ek2, xn2, xr, xi);
-  if constexpr (N > 8) householder_phase<T, N, 8>(ar, ai, s, lane, dk, ek2, xn2, xr, xi);
+  householder_phase<T, N, 0>(ar, ai, s, lane, n, dk, ek2, xn2, xr, xi);
+  if constexpr (N > 8) householder_phase<T, N, 8>(ar, ai, s, lane, n, dk, ek2, xn2, xr, xi);
   if constexpr (N > 16) {
-    householder_phase<T, N, 16>(ar, ai, s, lane, dk, ek2, xn2, xr, xi);
-    householder_phase<T, N, 24>(ar, ai, s, lane, dk, ek2, xn2, xr, xi);
+    householder_phase<T, N, 16>(ar, ai, s, lane, n, dk, ek2, xn2, xr, xi);
+    householder_phase<T, N, 24>(ar, ai, s, lane, n, dk, ek2, xn2, xr, xi);
   }
   if (lane == N - 1) dk = ar[N - 1];
   s.d[lane] = dk;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel
     const bool live = b < a.batch;
     T ar[N], ai[N];
     load_rows<T, N>(a, b, lane, live, ar, ai, s);
-    householder_tridiag<T, N>(ar, ai, s, lane);
+    householder_tridiag<T, N>(ar, ai, s, lane, n);
     if (MODE == 2) {
       if (live) {
         a.Dt[b * 32 + lane] = (double)s.d[lane];
