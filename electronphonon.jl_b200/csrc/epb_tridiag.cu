@@ -8,7 +8,7 @@
 // eigensolve; eigenvalues come from bisection on T.
 //
 // N lanes per matrix (N = 8, 16 or 32); lane i holds row i of the (zero-padded) N x N matrix in registers. Step k
-// (k = 0 .. N-3) reflects x = A[k+1:N, k] onto a multiple of e_1 with the Hermitian unitary
+// (k = 0 .. n-2) reflects x = A[k+1:N, k] onto a multiple of e_1 with the Hermitian unitary
 // P = I - beta u u^H, u = x + e^{i theta} ||x|| e_1 (theta = arg x_1), beta = 1 / (||x|| (||x|| + |x_1|)),
 // and updates the trailing block as A <- A - u w^H - w u^H with p = beta A u,
 // K = (beta / 2) u^H p (real), w = p - K u. The tridiagonal keeps d_k = A[k][k] and the squared
@@ -309,9 +309,9 @@ __device__ __forceinline__ int sturm_signs(const double* d, const double* e2, in
 
 // MODE 0: window band ranges from Sturm counts at the shifts; MODE 1: all eigenvalues; MODE 2: the
 // tridiagonal itself (d, e^2) for a later per-band bisection. N lanes per matrix. What bounds the FP64 reduction:
-// two warps per scheduler (128 registers hold a row of 32), each step a chain of two lane sums, two reciprocal
-// square roots and a division around 16 FP64 FMAs per column. Window counts of 98292 matrices of order 32:
-// 5.5 -> 4.1 ms (two blocks per SM, without the few spills: 4.7).
+// three warps per scheduler (a row of 32 takes 168 registers), each step a chain of two lane sums, two reciprocal
+// square roots and a division around 14 FP64 operations per column, and its broadcast reads of u and w. Window counts of
+// 98292 matrices of order 32: 5.5 -> 4.4 ms (two blocks per SM, without the few spills, a sixth more).
 template <typename T, int N, int MODE>
 __global__ void __launch_bounds__(32 * TRI_WARPS, TRI_MINB(T, N)) tridiag_kernel(TriArgs a) {
   constexpr int G = 32 / N;  // matrices per warp

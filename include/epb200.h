@@ -15,6 +15,12 @@
  *    inside the context (grown on demand, released by epb_destroy).
  *  - All work is stream-ordered on the context's stream; nothing synchronises unless stated. The
  *    caller synchronises (the reference's `synchronize(backend)`, src/common/gpu_utils.jl:60).
+ *    epb_set_stream orders nothing between the old stream and the new one. Large FP64 sums and products and FP64
+ *    eigensolves order what they keep in the context by themselves; other calls share workspaces, so that
+ *    the caller orders them when it moves a context between streams.
+ *  - FP64 results are accurate to a few eps whatever the batch, but which kernel forms them follows from its size: the
+ *    same point in lists of different lengths can differ in its last bits (and eigenvectors of a degenerate level
+ *    by a rotation).
  *  - Every function returns an int status (EPB_OK == 0) and never aborts or throws across the ABI;
  *    epb_last_error() gives a message for the calling thread's last failure.
  *  - Threading: one context per host thread, no internal locking (the reference's batched loop is
