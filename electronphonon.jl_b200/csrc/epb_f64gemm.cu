@@ -319,7 +319,7 @@ static int gemm_dispatch(epb_ctx* ctx, const F64GemmArgs& a) {
     if (a.serial && shapes[i].wk > 1) continue;
     const double bm = shapes[i].bm, bn = shapes[i].bn;
     const double waves = (double)cdiv(cdiv(a.M, shapes[i].bm) * cdiv(a.N, shapes[i].bn), ctx->sm_count);
-    const double c = waves * ((bm * bn + 128.0) * (double)a.K + 16.0 * bm * bn + 40.0 * bn * (a.L0 + a.L1 + a.L2));
+    const double c = waves * ((bm * bn + 128.0) * (double)std::max<int64_t>(a.K, 8) + 16.0 * bm * bn + 40.0 * bn * (a.L0 + a.L1 + a.L2));
     if (c < cost * 0.999) cost = c, best = i;
   }
   switch (best) {
