@@ -98,14 +98,19 @@ __global__ void __launch_bounds__(256) rq_mode_rotate_reg_kernel(const G* __rest
   }
 }
 
-// out = the mode rotation of g; out may not overlap g.
+// out = the mode rotation of g; out may not overlap g. With a single band the register kernel's loads are nm entries apart;
+// until the outputs fill the chip a thread per output is the faster one (6 modes, 343 Re, 6 q 7.0 against 8.3 us; 12 modes,
+// 2197 Re, 1 q 8.6 / 11.8; 12, 9261, 1, 111000 outputs 10.6 / 11.7; 12, 2197, 6, 158000 outputs 12.7 / 12.1).
 template <typename G>
 static int rq_mode_rotate(epb_ctx* ctx, const G* g, const double2* uph, int64_t nb, int64_t nm, int64_t nr, int64_t nq,
                           double2* out) {
   const int64_t tiles = cdiv(nb * nr, 256) * nq;
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)ctx->sm_count * 8));
+  const bool per_output = nm > 15 || (nb == 1 && nm > 3 && nm * nr * nq < 120000);
   prof_begin(ctx, EPB_PROF_RR_ROT);
-  if (nm <= 3)
+  if (per_output)
+    rq_mode_rotate_kernel<G><<<grid_oq(ctx, nb * nm * nr * nq), 256, 0, ctx->stream>>>(g, uph, nb, nm, nr, nq, out);
+  else if (nm <= 3)
     rq_mode_rotate_reg_kernel<G, 3><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
   else if (nm <= 6)
     rq_mode_rotate_reg_kernel<G, 6><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
@@ -113,10 +118,8 @@ static int rq_mode_rotate(epb_ctx* ctx, const G* g, const double2* uph, int64_t 
     rq_mode_rotate_reg_kernel<G, 9><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
   else if (nm <= 12)
     rq_mode_rotate_reg_kernel<G, 12><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
-  else if (nm <= 15)
-    rq_mode_rotate_reg_kernel<G, 15><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
   else
-    rq_mode_rotate_kernel<G><<<grid_oq(ctx, nb * nm * nr * nq), 256, 0, ctx->stream>>>(g, uph, nb, nm, nr, nq, out);
+    rq_mode_rotate_reg_kernel<G, 15><<<grid, 256, 0, ctx->stream>>>(g, uph, nb, (int)nm, nr, nq, out);
   prof_end(ctx);
   EPB_LAUNCH_CHECK();
   return EPB_OK;
