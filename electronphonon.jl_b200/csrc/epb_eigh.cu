@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(NT, MINB) eigh64_kernel(EighArgs a, unsigned l
     double tot = 0;
     for (int w = 0; w < NW; ++w) tot += red[w];
     const double thr = 2.220446049250313e-16 * sqrt(tot) / n, thr2 = thr * thr;
+    const bool bad = !isfinite(tot);  // an infinity or NaN in the matrix (nothing is rotated then): no states
     // Odd n: index n is an absent player whose pair never rotates; what its places in A hold meets no other element.
     const int m = (n + 1) & ~1, npair = m / 2, ng = NT / npair;
     const int i = tid % npair, g = tid / npair;  // this thread's pair of rows, and its share of the pairs of columns
@@ -273,7 +274,8 @@ __global__ void __launch_bounds__(NT, MINB) eigh64_kernel(EighArgs a, unsigned l
         const double ej = As[j + j * lda].x;
         rank += (ej < ei) || (ej == ei && j < i);
       }
-      if (a.E) a.E[eoff + rank] = a.mass ? (ei >= 0 ? sqrt(ei) : -sqrt(-ei)) : ei;
+      if (bad) rank = i;  // comparisons with NaN rank nothing
+      if (a.E) a.E[eoff + rank] = bad ? nan("") : a.mass ? (ei >= 0 ? sqrt(ei) : -sqrt(-ei)) : ei;
       // stash rank in the (now unused) imaginary part of the diagonal
       As[i + i * lda].y = (double)rank;
     }
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(NT, MINB) eigh64_kernel(EighArgs a, unsigned l
       for (int e = tid; e < n * n; e += NT) {
         const int row = e % n, col = e / n;
         const int rank = (int)As[col + col * lda].y;
-        double2 o = Vs[e];
+        double2 o = bad ? make_double2(nan(""), nan("")) : Vs[e];
         if (a.mass) {
           const double s = 1.0 / sqrt(a.mass[row]);
           o.x *= s;

@@ -543,13 +543,16 @@ __global__ void __launch_bounds__(128, NR > 12 ? 3 : 4) eigh16_fp64_kernel(Eigh1
     double nr2 = 0.0;
 #pragma unroll
     for (int i = 0; i < NR; ++i) nr2 += col[i].x * col[i].x + col[i].y * col[i].y;
-    const double inv = 1.0 / sqrt(nr2), lam = sqrt(nr2) - sigma;
+    // an infinity or NaN in the matrix: no states (comparisons with NaN would rank nothing)
+    const bool bad = !isfinite(f2);
+    const double inv = bad ? nan("") : 1.0 / sqrt(nr2), lam = bad ? nan("") : sqrt(nr2) - sigma;
     int rank = 0;
 #pragma unroll
     for (int k = 0; k < GL; ++k) {
       const double lk = __shfl_sync(0xffffffffu, lam, (lane & ~(GL - 1)) + k);
       rank += (k < n) && (lk < lam || (lk == lam && k < l));
     }
+    if (bad) rank = l;
     if (live && l < n) {
       if (a.E) a.E[b * n + rank] = a.mass ? (lam >= 0 ? sqrt(lam) : -sqrt(-lam)) : lam;
       if (a.U64) {
