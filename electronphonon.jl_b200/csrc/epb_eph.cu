@@ -6,8 +6,8 @@
 //  * rotations (ext/ElectronPhononCUDAExt.jl:146-201, src/wannier_to_bloch_batched.jl:442-455):
 //    T = ukq^dagger g (contract iw) and ep = T uph (contract jm), folding g2 = |ep|^2/(2 omega)
 //    into the same pass: epb_rot64.cu up to 15 modes and 32 bands where its cost is the lower one (rot64_pays); else,
-//    and with an output over an input, one CTA per q stages g(q), ukq(q), uph(q) in shared memory. The reference switches to two cuBLAS strided-batched
-//    GEMMs above nw*nm = 24 (wannier_to_bloch_batched.jl:406).
+//    and with an output over an input, one CTA per q stages g(q), ukq(q), uph(q) in shared memory. The reference
+//    switches to two cuBLAS strided-batched GEMMs above nw*nm = 24 (wannier_to_bloch_batched.jl:406).
 #include <algorithm>
 
 #include "epb_common.cuh"
